@@ -19,6 +19,13 @@
  * An engine is not thread-safe: one thread at a time per engine (the reference-
  * compatible layer serialises its calls per context with a mutex); different
  * engines may be used from different threads.
+ * Calls of one engine on several streams: evaluations (evolved state, energies,
+ * gradients) share the engine's state vectors, so the caller orders them; H products
+ * (aegpu_apply_dev without energy_dev) need no order among themselves or beside an
+ * evaluation, except that with as many alpha as beta electrons outside the tensor-core
+ * product they share the partial sums of the spin-flip test.  Calls recorded into a
+ * caller's own graph take the FP64 product kernels (a replay cannot be ordered with the
+ * engine's other calls); those that replay a graph of the engine cannot be recorded.
  */
 #ifndef AEGPU_H
 #define AEGPU_H
