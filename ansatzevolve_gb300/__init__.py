@@ -20,7 +20,7 @@ _LIB = None
 
 HAM_AUTO, HAM_STORED, HAM_ON_THE_FLY = 0, 1, 2
 TUNE_PASS_OPS, TUNE_CTAS_PER_SM, TUNE_OTF_THREADS, TUNE_SPMV_TPR, TUNE_PDL, TUNE_REUSE_HPSI, TUNE_FLIP = 1, 2, 3, 4, 5, 6, 7
-TUNE_HALF = 8
+TUNE_HALF, TUNE_TENSOR = 8, 9
 BASIS_FULL, BASIS_NUMBER, BASIS_SZ = 0, 1, 2
 PROP_HESSIAN, PROP_OVERLAP, PROP_HF_PATH = 1, 2, 4
 # rows of the properties table, in the reference's print order (tupsquantities.cpp:538-566)
@@ -74,6 +74,7 @@ def lib(build_if_missing=True):
         "aegpu_set_tuning": (ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int]),
         "aegpu_flip_status": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int)]),
         "aegpu_half_status": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int)]),
+        "aegpu_tensor_status": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int)]),
         "aegpu_half_info": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int64)]),
         "aegpu_get_tuning": (ctypes.c_int, [_P, ctypes.c_int]),
         "aegpu_io_dev": (ctypes.c_int, [_P, ctypes.POINTER(_P), ctypes.POINTER(_P), ctypes.POINTER(_P)]),
@@ -553,7 +554,7 @@ class Engine:
 
     def set_tuning(self, knob, value):
         """One knob (TUNE_*) where the engine accepts it at this point of its set-up
-        (TUNE_PDL, TUNE_REUSE_HPSI, TUNE_FLIP and TUNE_HALF at any time)."""
+        (TUNE_PDL, TUNE_REUSE_HPSI, TUNE_FLIP, TUNE_HALF and TUNE_TENSOR at any time)."""
         self._check(self.L.aegpu_set_tuning(self.h, knob, int(value)))
 
     def get_tuning(self, knob):
@@ -564,6 +565,12 @@ class Engine:
         half product."""
         u = np.zeros(self.nb, dtype=np.int32)
         self._check(self.L.aegpu_flip_status(self.h, iptr(u)))
+        return u.astype(bool)
+
+    def tensor_status(self):
+        """Per instance: True where the last H product ran on the tensor cores."""
+        u = np.zeros(self.nb, dtype=np.int32)
+        self._check(self.L.aegpu_tensor_status(self.h, iptr(u)))
         return u.astype(bool)
 
     def half_status(self):

@@ -73,9 +73,11 @@ bool tc_build(TcProduct &t, const TcBasis &B, const double *h1s, const double *g
 bool tc_alloc_workspace(TcProduct &t, int W, int max_inst, const TcAlloc &alloc, cudaStream_t s);
 // y = H x of ninst vectors of D * W doubles.  bad[b] != 0 after the stream reached this
 // point: instance b was left to the caller's other product (a value that is not finite
-// or out of the digits' range).  epart: ngx partial sums of <x|y> per instance
-// (nullable).  flip_tol2 < 0: do not use psi(a,b) = psi(b,a).  Returns kernel launches.
-int tc_apply(const TcProduct &t, const double *x, double *y, int ninst, const int *active, double flip_tol2, int *flip_used,
-             int *bad, double *epart, cudaStream_t s);
+// or out of the digits' range, or, with elements -- y goes to a caller who may look at single
+// elements -- a vector of too wide a range).  epart: ngx partial sums of <x|y> per instance
+// (nullable).  flip_tol2 < 0: do not use psi(a,b) = psi(b,a); flip_sums: its test's two
+// sums per instance, for the caller's other product (nullable).  Returns kernel launches.
+int tc_apply(const TcProduct &t, const double *x, double *y, int ninst, const int *active, bool elements, double flip_tol2,
+             int *flip_used, double *flip_sums, int *bad, double *epart, cudaStream_t s);
 
 }  // namespace ae
