@@ -64,10 +64,12 @@ using TcAlloc = std::function<void *(size_t bytes)>;
 bool tc_shape(TcProduct &t, const TcBasis &B, int sm_count, int smem_optin);
 // Workspace bytes of one instance.
 size_t tc_workspace(const TcProduct &t, int W);
+// Whether the integrals g2s of ntab Hamiltonians are finite and have the symmetry (pq|rs) = (qp|rs) = (pq|sr).
+bool tc_symmetric(int N, const double *g2s, int ntab);
 // String tables, digit tables of ntab Hamiltonians (host h1s/g2s, device copies d_h1/d_g2),
-// and the workspace for up to max_inst instances.  False (t.ok cleared): the integrals lack the
-// (pq|rs) = (qp|rs) = (pq|sr) symmetry, the digits' exactness bound does not hold, or an allocation
-// failed.  Values only (same shape): tables are rewritten in place.
+// of integrals that tc_symmetric takes.  False (t.ok cleared): the digits' exactness bound does not
+// hold, a same-spin element is not finite, or an allocation failed.  Values only (same shape):
+// tables are rewritten in place.
 bool tc_build(TcProduct &t, const TcBasis &B, const double *h1s, const double *g2s, const double *d_h1,
               const double *d_g2, const double *diag, int ntab, const TcAlloc &alloc, bool values_only, cudaStream_t s);
 bool tc_alloc_workspace(TcProduct &t, int W, int max_inst, const TcAlloc &alloc, cudaStream_t s);
