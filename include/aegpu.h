@@ -134,20 +134,21 @@ enum { AEGPU_TUNE_PASS_OPS = 1, AEGPU_TUNE_CTAS_PER_SM = 2, AEGPU_TUNE_OTF_THREA
        AEGPU_TUNE_PDL = 5, AEGPU_TUNE_REUSE_HPSI = 6, AEGPU_TUNE_FLIP = 7, AEGPU_TUNE_HALF = 8, AEGPU_TUNE_TENSOR = 9 };
 int aegpu_set_tuning(aegpu_engine *e, int knob, int value);
 int aegpu_get_tuning(const aegpu_engine *e, int knob);
-/* AEGPU_TUNE_TENSOR (1, the default, or 0; any time, it rebuilds the captured graphs): the
- * product of integral Hamiltonians of larger Sz sectors on the tensor cores, with the FP64
- * operands split into bf16 digits and integer sums.  Its error is the same for every element
- * of H x, about a third of the FP64 kernels' root mean square for a vector of one scale; an
- * element made of small elements of x alone has fewer correct bits than theirs.  Energies,
- * gradients, Hessians and eigenpairs are inner products over all elements and take it for any
- * vector; aegpu_apply_h and aegpu_apply_dev take it for vectors without a tail of small
- * elements (tested on the device: normal or uniform distributions pass, a state dominated by a
- * few determinants does not) and the FP64 kernels otherwise.  With 0 every product is theirs.
- * The environment variable AEGPU_TENSOR=0 keeps engines created afterwards from building its
- * tables (the knob then has no effect); AEGPU_TENSOR=1 builds them for every sector that
- * they can hold (a diagnostic switch).
- * used[b] = 1 where the engine's last H product of instance b ran on the tensor cores
- * (waits for it). */
+/* AEGPU_TUNE_TENSOR (1, the default, or 0; any time, it rebuilds the captured graphs): H products
+ * of integral Hamiltonians on the tensor cores, with the FP64 operands split into bf16 digits
+ * and integer sums, in sectors of at least 200 alpha and 40 beta strings and calls of at least
+ * 2e7 matrix elements over all their vectors.  The error is the same for every element of H x,
+ * for a vector of one scale about half of the FP64 kernels' root mean square; an element made of
+ * small elements of x alone has fewer correct bits than theirs.  Energies, gradients, Hessians
+ * and eigenpairs are inner products over all elements and take it for any vector; aegpu_apply_h
+ * and aegpu_apply_dev take it for vectors without a tail of small elements (tested on the
+ * device: normal or uniform distributions pass, a state dominated by a few determinants does
+ * not) and the FP64 kernels otherwise.  With 0 every product is theirs.  The environment
+ * variable AEGPU_TENSOR=0 keeps engines created afterwards from building its tables (the knob
+ * then has no effect); AEGPU_TENSOR=1 takes every sector that the tables can hold (a diagnostic
+ * switch).
+ * used[b] = 1 where the engine's last H product of instance b ran on the tensor cores (waits
+ * for it). */
 int aegpu_tensor_status(aegpu_engine *e, int *used);
 /* used[b] = 1 where the last energy evaluation's H psi of instance b took the spin-flip
  * half product, 0 where it took the full one (or did not test; masked instances keep
