@@ -6,7 +6,8 @@ knobs and keeps the fastest:
 
 * TUNE_PASS_OPS: excitations fused into one pass of the statevector (1..6; more per
   pass means fewer sweeps over HBM, but fewer commuting excitations to fill a pass);
-* TUNE_CTAS_PER_SM: CTAs per SM of the pass kernels (occupancy against tail effects);
+* TUNE_CTAS_PER_SM: CTAs per SM of the pass kernels (occupancy against tail effects; 4, the
+  default, includes the engine's choice by size for the adjoint passes);
 * TUNE_OTF_THREADS: threads per CTA of the on-the-fly H*psi kernel (one CTA per alpha
   string and chunk of beta strings);
 * TUNE_SPMV_TPR: threads per row of the stored-H product (0 = chosen by size).

@@ -94,7 +94,8 @@ int aegpu_set_ham_integrals(aegpu_engine *e, const double *h1, const double *g2,
 int aegpu_set_batch(aegpu_engine *e, int nb);
 /* Launch-shape knobs (picked by the autotuner, ansatzevolve_gb300/autotune.py):
  * excitations fused per pass (1..6; before aegpu_set_problem), CTAs per SM of the
- * pass kernels (1..64; before aegpu_set_problem), threads per CTA of the on-the-fly
+ * pass kernels (1..64; before aegpu_set_problem; 4, the default: 4, and 2 in the adjoint
+ * passes of real circuits where that gives a warp two to eight tasks), threads per CTA of the on-the-fly
  * H kernel (64..1024, multiple of 32; before the Hamiltonian; unset, 512, or as many as
  * fit in equal beta chunks of up to 1024 when the string tables leave room for only one
  * CTA per SM), threads per row of the
