@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kGramThreads) k_gram(const double *__restrict_
 }
 
 // C[i + j ldc] = alpha * sum over chunks (fixed order) of the partials, i <= j < V.  A CTA
-// sums 32 elements of pair blockIdx.y, eight threads each over an eighth of the chunks (a
+// sums 32 elements of pair blockIdx.x, eight threads each over an eighth of the chunks (a
 // thread per element: 62 us for 202 chunks; so: 17 us for 397).
 __global__ void __launch_bounds__(256) k_gram_finish(const double *__restrict__ partial, int nchunks, int npairs, int V, int W,
                                                      double alpha, double *__restrict__ Cre, double *__restrict__ Cim, int ldc)
@@ -152,15 +152,15 @@ __global__ void __launch_bounds__(256) k_gram_finish(const double *__restrict__ 
     constexpr int PP = kGramPanel * kGramPanel;
     __shared__ double part[8][32];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int rem = blockIdx.x * 32 + tx, w = rem / PP, e = rem % PP;
+    const int rem = blockIdx.y * 32 + tx, w = rem / PP, e = rem % PP;
     int I, J;
-    pair_of(blockIdx.y, I, J);
+    pair_of(blockIdx.x, I, J);
     const int i = I * kGramPanel + e % kGramPanel, j = J * kGramPanel + e / kGramPanel;
     const bool on = j < V && i <= j;
     double s = 0.0;
     if (on)
         for (int c = nchunks * ty / 8; c < nchunks * (ty + 1) / 8; ++c)
-            s += partial[((int64_t)c * npairs + blockIdx.y) * W * PP + rem];
+            s += partial[((int64_t)c * npairs + blockIdx.x) * W * PP + rem];
     part[ty][tx] = s;
     __syncthreads();
     if (ty || !on) return;
@@ -383,7 +383,8 @@ int gram_upper(const double *A, int64_t lda, const double *B, int64_t ldb, int64
         k_gram<1><<<grid, kGramThreads, 0, s>>>(A, lda, B, ldb, nrows, V, g.npairs, g.slabs_per_chunk, scratch);
     else
         k_gram<2><<<grid, kGramThreads, 0, s>>>(A, lda, B, ldb, nrows, V, g.npairs, g.slabs_per_chunk, scratch);
-    k_gram_finish<<<dim3(W * kGramPanel * kGramPanel / 32, g.npairs), 256, 0, s>>>(scratch, g.nchunks, g.npairs, V, W, alpha,
+    // pairs on grid.x: more than 65,535 of them from 23,105 columns on
+    k_gram_finish<<<dim3(g.npairs, W * kGramPanel * kGramPanel / 32), 256, 0, s>>>(scratch, g.nchunks, g.npairs, V, W, alpha,
                                                                                 Cre, Cim, ldc);
     return 2;
 }
