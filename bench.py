@@ -172,10 +172,9 @@ class ClockSampler:
                 "reasons": sorted(reasons)}
 
 
-def on_tensor_cores(strings):
-    """Whether H*psi of an integral Hamiltonian runs on the tensor cores (csrc/tensor.cu):
-    Sz sectors of at least 200 alpha strings."""
-    return strings >= 200 and os.environ.get("AEGPU_TENSOR") != "0"
+def on_tensor_cores(engine):
+    """Whether the engine's last H*psi ran on the tensor cores (csrc/tensor.cu), for every instance."""
+    return bool(engine.tensor_status().all())
 
 
 def tensor_roofline(elements, W, ms):
@@ -468,7 +467,7 @@ def batched_bench(stream, steps=10, warmup=3):
         # the class against the FP64 pipe: FP64 instructions of its evaluations (one DFMA
         # per matrix element, per amplitude-layer forward, two adjoint) over the measured
         # DFMA rate
-        fw = sum(e.fp64_work()[1:] if on_tensor_cores(math.comb(N, na)) else e.fp64_work())
+        fw = sum(e.fp64_work()[1:] if on_tensor_cores(e) else e.fp64_work())
         pc["fp64_instr_per_batch"] = int(fw * pc["instances"])
         pc["fp64_frac"] = fw * pc["instances"] / (pc["ms_per_batch"] / 1e3) / 1e12 / peak_t
     E, g = engines[0].io_get_results()
@@ -564,7 +563,7 @@ def aux_case_bench(n_orb, lucj, stream, steps=5, warmup=2):
                "config": workload_desc(D, pb["P"], len(pb["ops0"]), "regenerated on the fly"),
                "setup_s": setup_s, "passes": passes, "half_passes": half_passes,
                "phase_ms": {"evolve": ph[0], "hpsi_energy": ph[1], "adjoint": ph[2]},
-               "hpsi": tensor_roofline(fw[0] / W, W, ph[1]) if on_tensor_cores(int(round(D ** 0.5))) else
+               "hpsi": tensor_roofline(fw[0] / W, W, ph[1]) if on_tensor_cores(eng) else
                        {"fp64_instructions": int(fw[0]), "achieved_T_per_s": fw[0] / (ph[1] / 1e3) / 1e12,
                         "peak_T_per_s": peak_t, "frac": fw[0] / (ph[1] / 1e3) / 1e12 / peak_t,
                         "peak_source": "measured (aegpu_fp64_peak)"},
@@ -977,7 +976,7 @@ def main():
     # FP64-pipe roofline of the same step: FP64 instructions per evaluation against the
     # DFMA throughput measured on this device right now
     fw = eng.fp64_work()
-    tensor = on_tensor_cores(nA)
+    tensor = on_tensor_cores(eng)
     if tensor:  # the matrix elements' products are not on the FP64 pipe
         fw = (0,) + tuple(fw[1:])
     fw_h = fw[0]
