@@ -100,10 +100,9 @@ int aegpu_set_batch(aegpu_engine *e, int nb);
  * fit in equal beta chunks of up to 1024 when the string tables leave room for only one
  * CTA per SM), threads per row of the
  * stored-H product (1, 2, 4, 8; 0 = chosen by size; before the first evaluation),
- * programmatic dependent launch of the pass kernels (0 off, 1 on, -1 by size, the
- * default: on up to 2^19 amplitudes per launch; each pass's CTAs are scheduled while
- * the previous pass drains and wait on the device for its results; any time, it
- * rebuilds the captured graphs), reuse of H psi between an energy and a gradient at the
+ * programmatic dependent launch of the pass kernels (0 off; 1, the default, on; -1 is
+ * taken as 1; each pass's CTAs are scheduled while the previous pass drains and wait on
+ * the device for its results; any time, it rebuilds the captured graphs), reuse of H psi between an energy and a gradient at the
  * same angles (1, the default, or 0: the gradient recomputes H psi as the reference's
  * evolveDerivative does, fusedevolve.cpp:2292; the environment variable
  * AEGPU_REUSE_HPSI=0 sets 0 for engines created afterwards, e.g. the one behind the
