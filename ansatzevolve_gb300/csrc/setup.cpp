@@ -2,6 +2,7 @@
 #include "setup.h"
 
 #include <algorithm>
+#include <array>
 #include <numeric>
 #include <thread>
 
@@ -349,15 +350,6 @@ OrbitTables build_orbits(const Basis &B, const std::vector<ExcCode> &codes, int 
                     T.bits.push_back(orb[q]);
                 }
             }
-        const uint32_t per_tile = osz >= (uint32_t)kTileElems ? 1u : (uint32_t)kTileElems / osz;
-        for (uint32_t o = 0; o < g.n_orbits; o += per_tile) {
-            OrbitTile t{};
-            t.group = (uint32_t)T.groups.size();
-            t.orbit0 = o;
-            t.n_orbits = std::min(per_tile, g.n_orbits - o);
-            t.elem_off = g.idx_off + o * osz;
-            T.tiles.push_back(t);
-        }
         if (g.k <= (uint32_t)kMaxWarpLayers) {
             const uint32_t per_task = (uint32_t)kWarpElems / osz;
             for (uint32_t o = 0; o < g.n_orbits; o += per_task) {
@@ -521,10 +513,19 @@ extern "C" int aegpu_host_orbits(int nq, int kind, int ne, int na, int nb, int n
     for (int i = 0; i < nops; ++i) codes.push_back(ae::make_exc_code(ops[4 * i], ops[4 * i + 1], ops[4 * i + 2], ops[4 * i + 3]));
     ae::OrbitTables T = ae::build_orbits(B, codes, 2);
     if (!T.ok) return AEGPU_ERR_UNSUPPORTED;
+    // tiles: runs of whole orbits of one group with at most 4096 members (or one orbit), as
+    // (group, first orbit, orbits, first entry in the rank list)
+    std::vector<std::array<uint32_t, 4>> t;
+    for (size_t gi = 0; gi < T.groups.size(); ++gi) {
+        const ae::OrbitGroup &g = T.groups[gi];
+        const uint32_t per = std::max(1u, 4096u >> g.k);
+        for (uint32_t o = 0; o < g.n_orbits; o += per)
+            t.push_back({(uint32_t)gi, o, std::min(per, g.n_orbits - o), g.idx_off + (o << g.k)});
+    }
     const int64_t ci = *n_idx, cg = *n_groups, ct = *n_tiles;
     *n_idx = (int64_t)T.idx.size();
     *n_groups = (int64_t)T.groups.size();
-    *n_tiles = (int64_t)T.tiles.size();
+    *n_tiles = (int64_t)t.size();
     if (idx && ci >= *n_idx) std::copy(T.idx.begin(), T.idx.end(), idx);
     if (groups && cg >= *n_groups)
         for (size_t g = 0; g < T.groups.size(); ++g) {
@@ -534,12 +535,7 @@ extern "C" int aegpu_host_orbits(int nq, int kind, int ne, int na, int nb, int n
             groups[4 * g + 3] = T.groups[g].mask;
         }
     if (tiles && ct >= *n_tiles)
-        for (size_t t = 0; t < T.tiles.size(); ++t) {
-            tiles[4 * t] = T.tiles[t].group;
-            tiles[4 * t + 1] = T.tiles[t].orbit0;
-            tiles[4 * t + 2] = T.tiles[t].n_orbits;
-            tiles[4 * t + 3] = T.tiles[t].elem_off;
-        }
+        for (size_t i = 0; i < t.size(); ++i) std::copy(t[i].begin(), t[i].end(), tiles + 4 * i);
     return AEGPU_OK;
 }
 

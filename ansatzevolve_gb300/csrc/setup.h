@@ -116,24 +116,13 @@ bool exc_commutes(const Exc &x, const Exc &y);
 // root is the member that every active excitation maps to a larger bitstring.
 // Orbits are grouped by active mask; inside a group they are listed by ascending
 // root, each as 2^k ranks in hypercube order (bit i of the position = i-th active
-// excitation applied).  A tile is a run of whole orbits of one group with at most
-// kTileElems members: one CTA stages a tile in shared memory and applies all k
-// butterfly layers there, so the statevector crosses HBM once per block.
-constexpr int kTileElems = 4096;
-
+// excitation applied).
 struct OrbitGroup {
     uint32_t idx_off;    // first entry in the block's rank list
     uint32_t n_orbits;
     uint32_t k;          // active excitations per orbit
     uint32_t mask;       // block-local active mask
     int8_t slot[16];     // block-local excitation slot of layer i
-};
-
-struct OrbitTile {
-    uint32_t group;
-    uint32_t orbit0;
-    uint32_t n_orbits;
-    uint32_t elem_off;   // first entry in the block's rank list
 };
 
 // A warp task is a run of whole orbits of one group with at most 64 members (the
@@ -153,7 +142,6 @@ struct OrbitTables {
     std::vector<uint32_t> idx;        // ranks, grouped / ordered as described
     std::vector<uint32_t> bits;       // the determinants' bitstrings, parallel to idx
     std::vector<OrbitGroup> groups;
-    std::vector<OrbitTile> tiles;
     std::vector<WarpTask> wtasks;     // only when every orbit has <= 64 members
     uint64_t active = 0;              // number of determinants touched by the block
     uint64_t amp_layers = 0;          // sum over touched determinants of their active layers
