@@ -137,7 +137,7 @@ int aegpu_get_tuning(const aegpu_engine *e, int knob);
 /* AEGPU_TUNE_TENSOR (1, the default, or 0; any time, it rebuilds the captured graphs): H products
  * of integral Hamiltonians on the tensor cores, with the FP64 operands split into bf16 digits
  * and integer sums, in sectors of at least 200 alpha and 40 beta strings and calls of at least
- * 2e7 matrix elements over all their vectors.  The error is the same for every element of H x,
+ * 1.5e7 matrix elements over all their vectors.  The error is the same for every element of H x,
  * for a vector of one scale about half of the FP64 kernels' root mean square; an element made of
  * small elements of x alone has fewer correct bits than theirs.  Energies, gradients, Hessians
  * and eigenpairs are inner products over all elements and take it for any vector; aegpu_apply_h

@@ -26,8 +26,8 @@ def make(monkeypatch, tensor, N, na, nb, rows, cplx):
 
 
 @pytest.mark.parametrize("N,na,nb,rows,cplx,tensor", [
-    (12, 6, 1, 1, False, False), (12, 6, 1, 32, False, False), (13, 3, 12, 1, True, False), (10, 4, 3, 1, False, False),
-    (10, 4, 3, 4, False, True), (10, 4, 3, 1, True, True), (10, 5, 2, 1, False, False), (10, 5, 2, 12, False, True),
+    (12, 6, 1, 1, False, False), (12, 6, 1, 32, False, False), (13, 3, 12, 1, True, False), (13, 3, 2, 1, False, False),
+    (13, 3, 2, 2, False, True), (13, 3, 2, 1, True, True), (10, 4, 3, 1, False, True), (10, 5, 2, 1, False, False), (10, 5, 2, 12, False, True),
     (10, 5, 3, 1, False, True), (10, 5, 5, 1, False, True), (9, 5, 5, 16, False, False)])
 def test_rule(monkeypatch, N, na, nb, rows, cplx, tensor):
     e, ref = (make(monkeypatch, t, N, na, nb, rows, cplx) for t in (True, False))
