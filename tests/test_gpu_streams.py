@@ -99,3 +99,23 @@ def test_recorded_by_the_caller(monkeypatch, N, na, nb):
         assert torch.equal(E[1], E[2]) and torch.equal(g, h)
     e.close()
     ref.close()
+
+
+def test_an_engine_twice_in_a_group(monkeypatch):
+    """The evaluations of one engine in a group share its buffers: they run in turn."""
+    a, b = (make(monkeypatch, True, 10, 5, 5) for _ in range(2))
+    ang = np.random.default_rng(2).uniform(-0.3, 0.3, (2, a.nops))
+    want = [a.gradient(ang[0]), b.gradient(ang[1])]
+    group = ae.Group([a, b, a, a, b])
+    for e, x in ((a, ang[0]), (b, ang[1])):
+        e.io_put_angles(x)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        group.launch()
+        group.sync()
+        for e, (E, g) in ((a, want[0]), (b, want[1])):
+            E1, g1 = e.io_get_results()
+            assert np.array_equal(np.ravel(E1), np.ravel(E)) and np.array_equal(np.ravel(g1), np.ravel(g))
+    group.close()
+    a.close()
+    b.close()
